@@ -526,9 +526,7 @@ def _exact_spectrum(state, P, projection, unbinned):
         ks = torch.arange(int(math.sqrt(3) / 2 * P + 0.5) + 1, device="cuda") ** 2
         idx = (sq.double().sqrt() + 0.5).long()
     bins = torch.zeros(ks.numel(), device="cuda", dtype=torch.float64)
-    # on odd grids the corner modes lie past the last bin
-    keep = idx < ks.numel()
-    bins.index_add_(0, idx[keep], val.reshape(-1)[keep])
+    bins.index_add_(0, idx, val.reshape(-1))
     return {"bins": (bins / float(P) ** 6).cpu().numpy(), "ks": ks.cpu().numpy()}
 
 
