@@ -32,12 +32,14 @@ Twiddle *make_table(int P) {
 
 cudaError_t transform3(double2 *z, int n, int P, const Twiddle *table, cudaStream_t s) {
     const long long lines = (long long)n * P * P;
-    for (int axis = 0; axis < 3; ++axis)
-        if (!launch_small(P, z, lines, axis, table, s) &&
-            !launch_medium(P, z, lines, axis, table, s) &&
-            !launch_large(P, z, lines, axis, table, s))
-            return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    for (int axis = 0; axis < 3; ++axis) {
+        cudaError_t e = cudaErrorInvalidValue; /* P in none of the files */
+        if (!launch_small(P, z, lines, axis, table, s, &e) &&
+            !launch_medium(P, z, lines, axis, table, s, &e))
+            launch_large(P, z, lines, axis, table, s, &e);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 } // namespace fft

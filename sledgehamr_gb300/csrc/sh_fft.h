@@ -20,13 +20,14 @@ Twiddle *make_table(int P);
 cudaError_t transform3(double2 *z, int n, int P, const Twiddle *table, cudaStream_t s);
 
 /* One axis of a radix pair (the instantiations live in several files, which
- * compile in parallel); false when the pair is not in that file. */
+ * compile in parallel); false when the pair is not in that file, else *e is
+ * the launch's error. */
 bool launch_small(int P, double2 *z, long long lines, int axis, const Twiddle *table,
-                  cudaStream_t s);
+                  cudaStream_t s, cudaError_t *e);
 bool launch_medium(int P, double2 *z, long long lines, int axis, const Twiddle *table,
-                   cudaStream_t s);
+                   cudaStream_t s, cudaError_t *e);
 bool launch_large(int P, double2 *z, long long lines, int axis, const Twiddle *table,
-                  cudaStream_t s);
+                  cudaStream_t s, cudaError_t *e);
 
 } // namespace fft
 } // namespace sh

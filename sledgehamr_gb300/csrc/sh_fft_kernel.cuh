@@ -109,14 +109,22 @@ __global__ void __launch_bounds__(axis_threads<R1, R2>(), axis_threads<R1, R2>()
     }
 }
 
+/* A kernel's limit of dynamic shared memory belongs to the device that is
+ * current when it is set, and a process may have contexts on several: it is
+ * set at every launch that needs more than the 48 KB every device gives. */
 template <int R1, int R2>
-void launch_axis(double2 *z, long long lines, int axis, const Twiddle *table, cudaStream_t s) {
+cudaError_t launch_axis(double2 *z, long long lines, int axis, const Twiddle *table,
+                        cudaStream_t s) {
     constexpr size_t smem = axis_smem<R1, R2>();
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        axis_kernel<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    (void)attr; /* a failure shows as the launch's error */
+    if constexpr (smem + kLines * sizeof(int) > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(axis_kernel<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     axis_kernel<R1, R2><<<(int)((lines + kLines - 1) / kLines), axis_threads<R1, R2>(), smem, s>>>(
         z, lines, axis, table);
+    return cudaGetLastError();
 }
 
 } // namespace fft
