@@ -43,6 +43,7 @@
 #include "sh_bubbles.cuh"
 #include "sh_f32.cuh"
 #include "sh_fixed_stencil.h"
+#include "sh_halo.h"
 #include "sh_internal.h"
 #include "sledgehamr_gb300.h"
 
@@ -77,8 +78,6 @@ struct AxionArgs {
     int slot;               /* last stage writes slot 1 - slot = t + h */
     double h;
 };
-
-__device__ __forceinline__ int wrap(int a, int N) { return a < 0 ? a + N : (a >= N ? a - N : a); }
 
 
 template <class R>
@@ -150,15 +149,15 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 5 : 1) axion_rkn4_ker
     const R* Kin = STAGE == 1 ? a.K[0][0] : (STAGE == 2 ? a.K[1][0] : nullptr);
     const R* Kin2 = STAGE == 1 ? a.K[0][1] : (STAGE == 2 ? a.K[1][1] : nullptr);
 
-    /* plane element q of this thread: ring position and periodic source */
+    /* plane element q of this thread: ring position (-1: none) and periodic
+     * source */
     int ppos[NPL], pgx[NPL], pgy[NPL];
 #pragma unroll
     for (int q = 0; q < NPL; ++q) {
         const int p = tid + q * NT;
-        ppos[q] = p < W * HH ? p : -1;
-        const int px = p % W, py = p / W;
-        pgx[q] = wrap(tl.x0 - H + px, N);
-        pgy[q] = wrap(tl.y0 - H + py, N);
+        pgx[q] = halo_source(tl.x0 - H + p % W, N, H);
+        pgy[q] = halo_source(tl.y0 - H + p / W, N, H);
+        ppos[q] = p < W * HH && pgx[q] >= 0 && pgy[q] >= 0 ? p : -1;
     }
     R raw[NPL][6]; /* y0 (2), y0' (2), K (2) of the next plane */
     auto fetch = [&](int z) {
@@ -597,8 +596,9 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
 #pragma unroll
     for (int q = 0; q < NPL; ++q) {
         const int p = tid + q * NT;
-        ppos[q] = p < W * HH ? p : -1;
-        const int gx = wrap(tl.x0 - H + p % W, N), gy = wrap(tl.y0 - H + p / W, N);
+        const int gx = halo_source(tl.x0 - H + p % W, N, H);
+        const int gy = halo_source(tl.y0 - H + p / W, N, H);
+        ppos[q] = p < W * HH && gx >= 0 && gy >= 0 ? p : -1;
         pxy[q] = (long long)gy * N + gx;
     }
     R raw[NPL][NC];
