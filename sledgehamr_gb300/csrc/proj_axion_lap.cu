@@ -1,4 +1,5 @@
 /* AxionStringsLap1/2/3 project kernels (projects/AxionStringsLap). */
+#define SH_STAGE_CONSTANTS /* the registrations below name StageParams */
 #include "../projects/AxionStringsLap/AxionStringsLap.h"
 #include "sh_stage.cuh"
 SH_DEFINE_PROJECT_OPTIONS(AxionStringsLap1, ::AxionStringsLap1, false, 1, true,

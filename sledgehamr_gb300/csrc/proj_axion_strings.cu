@@ -1,4 +1,5 @@
 /* AxionStrings project kernels (hooks in projects/AxionStrings). */
+#define SH_STAGE_CONSTANTS /* the registrations below name StageParams */
 #include "../projects/AxionStrings/setup.h"
 #include "../projects/AxionStrings/kernels_rhs.h"
 #include "../projects/AxionStrings/kernels_tagging.h"

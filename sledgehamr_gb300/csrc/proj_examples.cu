@@ -1,4 +1,5 @@
 /* MinimalExample and NextToMinimalExample project kernels. */
+#define SH_STAGE_CONSTANTS /* the registrations below name StageParams */
 #include "../projects/MinimalExample/MinimalExample.h"
 #include "../projects/NextToMinimalExample/NextToMinimalExample.h"
 #include "sh_stage.cuh"

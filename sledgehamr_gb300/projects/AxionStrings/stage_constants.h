@@ -9,6 +9,13 @@
  * cell and stage with them, 11 without, on the 128^3 level).  The potential
  * takes three FP64 operations per cell instead of five as written above;
  * v0 = -v2 exactly for c = 0.
+ *
+ * The entries are written for projects registered with a StageParams function
+ * alone, so the hooks read them only in a translation unit that defines
+ * SH_STAGE_CONSTANTS and registers its projects that way (the shipped
+ * csrc/proj_*.cu).  Everywhere else - a project that calls a shipped Rhs, one
+ * registered with SH_DEFINE_PROJECT, a kernel of one's own - they form the
+ * constants themselves from the time and the project's parameters.
  */
 #ifndef SH_PROJECTS_AXION_STRINGS_STAGE_CONSTANTS_H_
 #define SH_PROJECTS_AXION_STRINGS_STAGE_CONSTANTS_H_
@@ -36,11 +43,11 @@ inline void store_constants(double *params, double eta, double lambda, double c)
     params[kFirst + 2] = s.v0;
 }
 
-/* The constants inside a hook: those of the launch on the device, formed
- * from lambda and c in host builds of the hook. */
+/* The constants inside a hook: those of the launch where it brings them,
+ * else formed from the time, lambda and c. */
 AMREX_GPU_HOST_DEVICE AMREX_FORCE_INLINE StageConstants constants(const double *params, double eta,
                                                                   double lambda, double c) {
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDA_ARCH__) && defined(SH_STAGE_CONSTANTS)
     return StageConstants{params[kFirst], params[kFirst + 1], params[kFirst + 2]};
 #else
     return make_constants(eta, lambda, c);
