@@ -258,7 +258,8 @@ SH_API int sh_level_rhs(sh_ctx *ctx, sh_level *level, int which, double time, in
  * covering its whole cubic periodic domain: the output function per cell,
  * its R2C FFT, and per bin of the sorted unique k^2 (as sh_spectrum_bins)
  * the sum of multpl |F|^2 times t / (N^6 dk), dk = 2 pi / (N dx), t the
- * level's SH_NEW time, multpl = 1 on the x planes 0 and N/2, else 2. */
+ * level's SH_NEW time, multpl = 1 on the x planes 0 and (N even) N/2, else
+ * 2. */
 SH_API int sh_scalar_spectrum(sh_ctx *ctx, const sh_level *level, int fn, int comp, double dx,
                               double *bins_out, long long *ks_out, int max_bins, int *nbins);
 /* Projection::Compute / Add (source/output_types/projection.cpp:10-118):

@@ -31,34 +31,12 @@
 #include <functional>
 #include <new>
 
-#ifdef _OPENMP
-#include <omp.h>
-#endif
-
 #include "sh_fft.cuh"
 #include "sh_gw.h"
+#include "sh_gw_bins.h"
 #include "sledgehamr_gb300.h"
 
 namespace sh {
-
-std::vector<long long> unique_k2_host(int dim) {
-    std::vector<long long> sq;
-    for (int a = 0; a < dim; ++a) {
-        long long f = a < (dim + 1) / 2 ? a : a - dim;
-        sq.push_back(f * f);
-    }
-    std::sort(sq.begin(), sq.end());
-    sq.erase(std::unique(sq.begin(), sq.end()), sq.end());
-    const long long maxs = 3 * sq.back();
-    std::vector<char> hit((size_t)maxs + 1, 0);
-    for (long long x : sq)
-        for (long long y : sq)
-            for (long long z : sq) hit[(size_t)(x + y + z)] = 1;
-    std::vector<long long> out;
-    for (long long v = 0; v <= maxs; ++v)
-        if (hit[(size_t)v]) out.push_back(v);
-    return out;
-}
 
 std::vector<double> index_to_k_host(int N, int type) {
     std::vector<double> r(N);
@@ -382,7 +360,8 @@ __global__ void scalar_power_kernel(const double2 *F, int P, double *out) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
          e += (long long)gridDim.x * blockDim.x) {
         const int a = (int)(e % H);
-        const double multpl = (a == 0 || a == P / 2) ? 1. : 2.;
+        /* the x planes that are their own mirror image count once */
+        const double multpl = (a == 0 || 2 * a == P) ? 1. : 2.;
         const double2 z = F[e];
         const double absF = sqrt(__dadd_rn(__dmul_rn(z.x, z.x), __dmul_rn(z.y, z.y)));
         out[e] = multpl * absF * absF;
@@ -415,69 +394,12 @@ void GwCache::prepare(int P, int unbinned, int projection_type) {
     g.unbinned = unbinned;
     g.projection_type = projection_type;
     g.used = clock;
-    const int H = P / 2 + 1;
-    const long long ncell = (long long)H * P * P;
-    if (unbinned) {
-        g.ks = unique_k2_host(P);
-    } else {
-        for (int k = 0; k <= std::sqrt(3.) / 2. * static_cast<double>(P) + .5; ++k)
-            g.ks.push_back((long long)k * k);
-    }
-    const int nb = (int)g.ks.size();
-    const long long maxsq = 3LL * (P / 2) * (P / 2);
-    std::vector<int> lut((size_t)maxsq + 1, -1);
-    if (unbinned) {
-        for (int q = 0; q < nb; ++q) lut[(size_t)g.ks[q]] = q;
-    } else {
-        for (long long sq = 0; sq <= maxsq; ++sq) {
-            long long r = (long long)std::llround(std::sqrt((double)sq));
-            /* round(sqrt(sq)) == r  <=>  r^2 - r < sq <= r^2 + r */
-            while (r * r + r < sq) ++r;
-            while (r > 0 && r * r - r >= sq) --r;
-            lut[(size_t)sq] = (int)r;
-        }
-    }
-    auto bin_of = [&](long long e) {
-        const int a = (int)(e % H), b = (int)((e / H) % P), c = (int)(e / ((long long)H * P));
-        const long long li = a >= P / 2 ? a - P : a;
-        const long long lj = b >= P / 2 ? b - P : b;
-        const long long lk = c >= P / 2 ? c - P : c;
-        return lut[(size_t)(li * li + lj * lj + lk * lk)];
-    };
-    /* stable counting sort over contiguous chunks of cells, one per thread */
-    int nt = 1;
-#ifdef _OPENMP
-    nt = std::max(1, std::min(omp_get_max_threads(), 64));
-#endif
-    const long long chunk = (ncell + nt - 1) / nt;
-    std::vector<long long> cnt((size_t)nt * nb, 0);
-#pragma omp parallel for num_threads(nt) schedule(static, 1)
-    for (int t = 0; t < nt; ++t) {
-        long long *c = cnt.data() + (size_t)t * nb;
-        const long long e1 = std::min(ncell, (t + 1) * chunk);
-        for (long long e = t * chunk; e < e1; ++e) c[bin_of(e)]++;
-    }
-    std::vector<long long> off(nb + 1, 0);
-    for (int q = 0; q < nb; ++q) {
-        long long run = off[q];
-        for (int t = 0; t < nt; ++t) {
-            const long long c = cnt[(size_t)t * nb + q];
-            cnt[(size_t)t * nb + q] = run; /* start of thread t's cells in bin q */
-            run += c;
-        }
-        off[q + 1] = run;
-    }
-    std::vector<int> cells((size_t)ncell);
-#pragma omp parallel for num_threads(nt) schedule(static, 1)
-    for (int t = 0; t < nt; ++t) {
-        long long *pos = cnt.data() + (size_t)t * nb;
-        const long long e1 = std::min(ncell, (t + 1) * chunk);
-        for (long long e = t * chunk; e < e1; ++e) cells[(size_t)pos[bin_of(e)]++] = (int)e;
-    }
+    const BinLists lists = bin_lists(P, unbinned != 0);
+    g.ks = lists.ks;
     std::vector<double> itk = index_to_k_host(P, projection_type);
     std::vector<float> itk32(itk.begin(), itk.end());
-    if (cudaMalloc(&g.d_off, off.size() * sizeof(long long)) != cudaSuccess ||
-        cudaMalloc(&g.d_cells, cells.size() * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc(&g.d_off, lists.off.size() * sizeof(long long)) != cudaSuccess ||
+        cudaMalloc(&g.d_cells, lists.cells.size() * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&g.d_itk, itk.size() * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&g.d_itk32, itk32.size() * sizeof(float)) != cudaSuccess) {
         cudaGetLastError();
@@ -487,8 +409,8 @@ void GwCache::prepare(int P, int unbinned, int projection_type) {
         cudaFree(g.d_itk32);
         throw std::bad_alloc();
     }
-    cudaMemcpy(g.d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    cudaMemcpy(g.d_cells, cells.data(), cells.size() * sizeof(int), cudaMemcpyHostToDevice);
+    cudaMemcpy(g.d_off, lists.off.data(), lists.off.size() * sizeof(long long), cudaMemcpyHostToDevice);
+    cudaMemcpy(g.d_cells, lists.cells.data(), lists.cells.size() * sizeof(int), cudaMemcpyHostToDevice);
     cudaMemcpy(g.d_itk, itk.data(), itk.size() * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(g.d_itk32, itk32.data(), itk32.size() * sizeof(float), cudaMemcpyHostToDevice);
     bins.push_back(std::move(g));
@@ -675,7 +597,7 @@ cudaError_t scalar_spectrum_packed(GwCache &cache, cudaStream_t stream, int P, d
     }
     cufftSetStream(plan, stream);
     double *real = scratch;
-    double2 *cplx = (double2 *)(scratch + nreal);
+    double2 *cplx = (double2 *)(scratch + nreal + nreal % 2); /* 16-byte aligned */
     double *vals = (double *)(cplx + ncplx);
     cudaMemsetAsync(real, 0, nreal * sizeof(double), stream);
     pack(real);

@@ -63,7 +63,6 @@ struct GwCache {
     void release();
 };
 
-std::vector<long long> unique_k2_host(int dim);
 std::vector<double> index_to_k_host(int N, int type);
 size_t gw_scratch_bytes(int N, int zero_padding);
 /* Scalar power spectrum of one P^3 real field that `pack(real)` writes into
