@@ -34,15 +34,14 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <functional>
 #include <new>
-#include <queue>
 #include <string>
 #include <vector>
 
 #include "sh_bubbles.cuh"
 #include "sh_f32.cuh"
 #include "sh_fixed_stencil.h"
+#include "sh_fuse_plan.h"
 #include "sh_halo.h"
 #include "sh_internal.h"
 #include "sledgehamr_gb300.h"
@@ -351,13 +350,6 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 5 : 1) axion_rkn4_ker
  * packed FP32 instructions measured the same).  Per step, FP32 + Kahan: one
  * 256^3 realisation 560 -> 285 us, a mix of eight from 32^3 to 128^3 262 ->
  * 127 us. */
-constexpr int kFuseSide = 32, kFuseHalo = 3, kFuseOut = kFuseSide - 2 * kFuseHalo;
-
-struct FusedTile {
-    int r;
-    int x0, y0, z0, w, h, nz;
-};
-
 constexpr size_t fused_smem() {
     /* stage positions [2][3] and momenta [4] of a plane of threads, pairs */
     return (size_t)(2 * 3 + 4) * kFuseSide * kFuseSide * sizeof(float2);
@@ -1157,58 +1149,16 @@ bool fused_steps(const sh_ensemble *E) {
     return E->family == SH_FAMILY_AXION_LAP1 && E->esize == 4;
 }
 
-/* Tiles of the fused kernel, longest first: every realisation cut into equal
- * columns of at most kFuseOut cells a side and into the depth (equal parts of
- * the largest realisation's planes) whose tiles end first when the SMs take
- * them in order, one block each.  A tile takes its rows with halo times its
- * planes with halo and two more for its start; on a mix of 32^3 to 128^3
- * boxes that predicts depths 16 / 26 / 32 / 43 / 64 within 2 % (165 / 135 /
- * 163 / 128 / 152 us per step). */
 void build_fused(sh_ensemble *E) {
-    auto cuts = [](int n, int most) { return (n + most - 1) / most; };
-    int dev = 0, nsm = 0, top = 0;
+    int dev = 0, nsm = 0;
     fck(cudaGetDevice(&dev), "device");
     fck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev), "SM count");
-    for (const RealDesc &d : E->desc)
-        if (d.active) top = std::max(top, d.N);
-    auto cost = [](const FusedTile &t) {
-        return (long long)(t.h + 2 * kFuseHalo) * (t.nz + 2 * kFuseHalo + 2);
-    };
-    std::vector<FusedTile> best, t;
-    long long least = 0;
-    for (int parts = 1; parts <= 16 && top > 0; ++parts) {
-        const int depth = cuts(top, parts);
-        if (parts > 1 && depth < 8) break;
-        t.clear();
-        for (int r = 0; r < E->nreal; ++r) {
-            if (!E->desc[r].active) continue;
-            const int N = E->desc[r].N;
-            const int w = cuts(N, cuts(N, kFuseOut)), nz = cuts(N, cuts(N, depth));
-            for (int z = 0; z < N; z += nz)
-                for (int y = 0; y < N; y += w)
-                    for (int x = 0; x < N; x += w)
-                        t.push_back(FusedTile{r, x, y, z, std::min(w, N - x), std::min(w, N - y),
-                                              std::min(nz, N - z)});
-        }
-        std::stable_sort(t.begin(), t.end(), [&](const FusedTile &a, const FusedTile &b) {
-            return cost(a) > cost(b);
-        });
-        std::priority_queue<long long, std::vector<long long>, std::greater<long long>> sm;
-        for (int q = 0; q < nsm; ++q) sm.push(0);
-        long long end = 0;
-        for (const FusedTile &q : t) {
-            const long long e = sm.top() + cost(q);
-            sm.pop();
-            sm.push(e);
-            end = std::max(end, e);
-        }
-        if (best.empty() || end < least) {
-            least = end;
-            best.swap(t);
-        }
-    }
-    upload_table(best, E->d_ftiles, E->ftiles_cap, est(E), "fused tile table");
-    E->ftiles.swap(best);
+    std::vector<FusedMember> members;
+    for (int r = 0; r < E->nreal; ++r)
+        if (E->desc[r].active) members.push_back(FusedMember{r, E->desc[r].N});
+    std::vector<FusedTile> t = plan_fused(members, nsm);
+    upload_table(t, E->d_ftiles, E->ftiles_cap, est(E), "fused tile table");
+    E->ftiles.swap(t);
     E->ftiles_stale = false;
 }
 
