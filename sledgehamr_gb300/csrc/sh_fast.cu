@@ -344,22 +344,22 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 5 : 1) axion_rkn4_ker
  * that a plane takes one barrier.  The arithmetic and its rounding are those
  * of axion_rkn4_kernel, stage by stage: the same bits.
  *
- * kFuseSide x kFuseSide threads, so up to kFuseOut = 26 x 26 cells a block
- * and one block per SM; 32 x 24 threads measured 11 %, two blocks of 32 x 16
- * 8 % slower at 256^3.  Bound by instruction issue (77 % of the slots; sm_100's
+ * 32 x 32 threads, so up to 26 x 26 cells a block and one block per SM (16 x
+ * 16 for members of up to 10^3 cells, sh_fuse_plan.h); 32 x 24 threads measured
+ * 11 %, two blocks of 32 x 16 8 % slower at 256^3.  Bound by instruction issue (77 % of the slots; sm_100's
  * packed FP32 instructions measured the same).  Per step, FP32 + Kahan: one
  * 256^3 realisation 560 -> 285 us, a mix of eight from 32^3 to 128^3 262 ->
  * 127 us. */
-constexpr size_t fused_smem() {
+constexpr size_t fused_smem(int side) {
     /* stage positions [2][3] and momenta [4] of a plane of threads, pairs */
-    return (size_t)(2 * 3 + 4) * kFuseSide * kFuseSide * sizeof(float2);
+    return (size_t)(2 * 3 + 4) * side * side * sizeof(float2);
 }
 
-template <bool KAHAN>
-__global__ void __launch_bounds__(kFuseSide *kFuseSide, 1)
+template <bool KAHAN, int SIDE>
+__global__ void __launch_bounds__(SIDE *SIDE, fused_blocks(SIDE))
     axion_rkn4_fused_kernel(const __grid_constant__ AxionArgs<float> a,
                             const FusedTile *__restrict__ tiles) {
-    constexpr int NT = kFuseSide * kFuseSide;
+    constexpr int NT = SIDE * SIDE;
     extern __shared__ float2 fsm[];
     float2(*pos)[3][NT] = reinterpret_cast<float2(*)[3][NT]>(fsm);        /* [2] */
     float2(*mom)[NT] = reinterpret_cast<float2(*)[NT]>(fsm + 2 * 3 * NT); /* [4] */
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kFuseSide *kFuseSide, 1)
     const FusedTile tl = tiles[blockIdx.x];
     const RealDesc d = a.desc[tl.r];
     const int N = d.N;
-    const int tx = threadIdx.x, ty = threadIdx.y, id = ty * kFuseSide + tx;
+    const int tx = threadIdx.x, ty = threadIdx.y, id = ty * SIDE + tx;
     if (id == 0) {
         const double hh = a.h * a.h;
         const double t0 = a.time[a.slot];
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(kFuseSide *kFuseSide, 1)
                        int stage) {
         const float friction = kc[4 + stage];
         const float v = f32::potential(c.x, c.y, lam, kc[7 + stage], cst);
-        const float2 xp = S[id + 1], xm = S[id - 1], yp = S[id + kFuseSide], ym = S[id - kFuseSide];
+        const float2 xp = S[id + 1], xm = S[id - 1], yp = S[id + SIDE], ym = S[id - SIDE];
         return make_float2(
             f32::accel(m.x, f32::lap7(c.x, xp.x, xm.x, yp.x, ym.x, up.x, dn.x, inv), c.x, v,
                        friction),
@@ -977,6 +977,7 @@ struct sh_ensemble {
     std::vector<FusedTile> ftiles;
     FusedTile *d_ftiles = nullptr;
     size_t ftiles_cap = 0;
+    int fuse_side = kFuseSide; /* threads a side of its blocks */
     bool ftiles_stale = true; /* the realisations changed since they were built */
     /* pools: capacity in cells of every array and the free extents
      * (offset -> length) */
@@ -1156,9 +1157,10 @@ void build_fused(sh_ensemble *E) {
     std::vector<FusedMember> members;
     for (int r = 0; r < E->nreal; ++r)
         if (E->desc[r].active) members.push_back(FusedMember{r, E->desc[r].N});
-    std::vector<FusedTile> t = plan_fused(members, nsm);
-    upload_table(t, E->d_ftiles, E->ftiles_cap, est(E), "fused tile table");
-    E->ftiles.swap(t);
+    FusedPlan plan = plan_fused(members, nsm);
+    upload_table(plan.tiles, E->d_ftiles, E->ftiles_cap, est(E), "fused tile table");
+    E->ftiles.swap(plan.tiles);
+    E->fuse_side = plan.side;
     E->ftiles_stale = false;
 }
 
@@ -1306,9 +1308,13 @@ void step_impl(sh_ensemble *E, const std::vector<void *> &in, const std::vector<
         }
         if (E->family == SH_FAMILY_AXION_LAP1) {
             if constexpr (sizeof(R) == 4) {
-                axion_rkn4_fused_kernel<KAHAN>
-                    <<<(int)E->ftiles.size(), dim3(kFuseSide, kFuseSide), fused_smem(), s>>>(
-                        a, E->d_ftiles);
+                const int n = (int)E->ftiles.size(), side = E->fuse_side;
+                if (side == kFuseSide)
+                    axion_rkn4_fused_kernel<KAHAN, kFuseSide>
+                        <<<n, dim3(side, side), fused_smem(side), s>>>(a, E->d_ftiles);
+                else
+                    axion_rkn4_fused_kernel<KAHAN, kFuseSmall>
+                        <<<n, dim3(side, side), fused_smem(side), s>>>(a, E->d_ftiles);
             } else {
                 axion_rkn4_kernel<R, 1, 0, KAHAN><<<nt, block, 0, s>>>(a);
                 axion_rkn4_kernel<R, 1, 1, KAHAN><<<nt, block, 0, s>>>(a);
@@ -1415,8 +1421,9 @@ void set_smem_limits() {
     fck(cudaFuncSetAttribute(T::axion_rkn4_tma_kernel<2, 0, true>, dyn, t2), "smem limit");
     fck(cudaFuncSetAttribute(T::axion_rkn4_tma_kernel<2, 1, true>, dyn, t2), "smem limit");
     fck(cudaFuncSetAttribute(T::axion_rkn4_tma_kernel<2, 2, true>, dyn, t2), "smem limit");
-    fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<true>, dyn, (int)fused_smem()), "smem limit");
-    fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<false>, dyn, (int)fused_smem()), "smem limit");
+    const int fsm = (int)fused_smem(kFuseSide); /* kFuseSmall needs no attribute */
+    fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<true, kFuseSide>, dyn, fsm), "smem limit");
+    fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<false, kFuseSide>, dyn, fsm), "smem limit");
     const int shf = (int)fopt_smem<float>();
     const int shd = (int)fopt_smem<double>();
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;

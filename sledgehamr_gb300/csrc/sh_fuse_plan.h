@@ -11,9 +11,14 @@
 namespace sh {
 namespace fast {
 
-/* A block's threads along x and y, one column each; the columns of halo on
- * each side that the three stages use up; the columns left. */
-constexpr int kFuseSide = 32, kFuseHalo = 3, kFuseOut = kFuseSide - 2 * kFuseHalo;
+/* A block has side x side threads, one column each, of which the three stages
+ * use up kFuseHalo on each side.  One block of side 32 fills an SM.  Members
+ * of up to 10^3 cells leave most of such a block idle and take side 16, four
+ * blocks per SM: 2000 members of 8^3 take 57 us per step against 140, FP32 + Kahan
+ * (127 with the stages launched one by one). */
+constexpr int kFuseSide = 32, kFuseSmall = 16, kFuseHalo = 3;
+constexpr int fused_out(int side) { return side - 2 * kFuseHalo; } /* columns left */
+constexpr int fused_blocks(int side) { return side == kFuseSmall ? 4 : 1; } /* per SM */
 
 struct FusedTile {
     int r;
@@ -30,10 +35,15 @@ struct FusedMember {
     int r, N; /* slot and cells a side */
 };
 
+struct FusedPlan {
+    int side = kFuseSide;
+    std::vector<FusedTile> tiles;
+};
+
 /* Tiles of the members, longest first: every member cut into equal columns of
- * at most kFuseOut cells a side and into the depth (equal parts of the largest
- * member's planes) whose tiles end first when nsm SMs take them in order, one
- * block each.  On a mix of 32^3 to 128^3 boxes the costs predict depths 16 /
+ * at most fused_out cells a side and into the depth (equal parts of the largest
+ * member's planes) whose tiles end first when nsm SMs take them in order, as
+ * many at a time as an SM holds blocks.  On a mix of 32^3 to 128^3 boxes the costs predict depths 16 /
  * 26 / 32 / 43 / 64 within 2 % (165 / 135 / 163 / 128 / 152 us per step).
  *
  * A pool plans at every admission and release, so a depth is tried on the
@@ -42,12 +52,15 @@ struct FusedMember {
  * halo, so that a pool of many tiles tries one or two of the sixteen): 24
  * members of 128^3 are planned in 0.02 ms, against 5.4 with every depth's
  * tiles listed and sorted. */
-inline std::vector<FusedTile> plan_fused(const std::vector<FusedMember> &members, int nsm) {
+inline FusedPlan plan_fused(const std::vector<FusedMember> &members, int nsm) {
     auto cuts = [](int n, int most) { return (n + most - 1) / most; };
     std::map<int, int> sizes; /* members by size */
     for (const FusedMember &m : members) ++sizes[m.N];
-    if (sizes.empty()) return {};
+    FusedPlan plan;
+    if (sizes.empty()) return plan;
     const int top = sizes.rbegin()->first;
+    if (top <= fused_out(kFuseSmall)) plan.side = kFuseSmall;
+    const int most = fused_out(plan.side), slots = nsm * fused_blocks(plan.side);
     int best = 0;
     long long least = 0;
     for (int parts = 1; parts <= 16; ++parts) {
@@ -55,8 +68,9 @@ inline std::vector<FusedTile> plan_fused(const std::vector<FusedMember> &members
         if (parts > 1 && depth < 8) break;
         std::map<long long, long long, std::greater<long long>> tiles; /* number by cost */
         long long total = 0;
-        for (const auto &[N, n] : sizes) {
-            const int w = cuts(N, cuts(N, kFuseOut)), nz = cuts(N, cuts(N, depth));
+        for (const auto &size : sizes) {
+            const int N = size.first, n = size.second;
+            const int w = cuts(N, cuts(N, most)), nz = cuts(N, cuts(N, depth));
             const int cols = cuts(N, w), layers = cuts(N, nz);
             /* rows and planes of the last tile along y and z */
             const int hl = N - (cols - 1) * w, nl = N - (layers - 1) * nz;
@@ -70,9 +84,9 @@ inline std::vector<FusedTile> plan_fused(const std::vector<FusedMember> &members
             add(w, nl, cols - 1);
             add(hl, nl, 1);
         }
-        if (best != 0 && std::max((total + nsm - 1) / nsm, tiles.begin()->first) >= least) continue;
+        if (best != 0 && std::max((total + slots - 1) / slots, tiles.begin()->first) >= least) continue;
         std::priority_queue<long long, std::vector<long long>, std::greater<long long>> sm;
-        for (int q = 0; q < nsm; ++q) sm.push(0);
+        for (int q = 0; q < slots; ++q) sm.push(0);
         long long end = 0;
         for (const auto &[cost, count] : tiles)
             for (long long q = 0; q < count; ++q) {
@@ -86,10 +100,10 @@ inline std::vector<FusedTile> plan_fused(const std::vector<FusedMember> &members
             best = depth;
         }
     }
-    std::vector<FusedTile> t;
+    std::vector<FusedTile> &t = plan.tiles;
     for (const FusedMember &m : members) {
         const int N = m.N;
-        const int w = cuts(N, cuts(N, kFuseOut)), nz = cuts(N, cuts(N, best));
+        const int w = cuts(N, cuts(N, most)), nz = cuts(N, cuts(N, best));
         for (int z = 0; z < N; z += nz)
             for (int y = 0; y < N; y += w)
                 for (int x = 0; x < N; x += w)
@@ -99,7 +113,7 @@ inline std::vector<FusedTile> plan_fused(const std::vector<FusedMember> &members
     std::stable_sort(t.begin(), t.end(), [](const FusedTile &a, const FusedTile &b) {
         return fused_cost(a.h, a.nz) > fused_cost(b.h, b.nz);
     });
-    return t;
+    return plan;
 }
 
 } // namespace fast

@@ -8,7 +8,8 @@
 
 using namespace sh::fast;
 
-static std::vector<FusedTile> exhaustive(const std::vector<FusedMember> &members, int nsm) {
+static std::vector<FusedTile> exhaustive(const std::vector<FusedMember> &members, int nsm,
+                                         int most) {
     auto cuts = [](int n, int most) { return (n + most - 1) / most; };
     std::vector<FusedTile> best;
     long long least = 0;
@@ -20,7 +21,7 @@ static std::vector<FusedTile> exhaustive(const std::vector<FusedMember> &members
         std::vector<FusedTile> t;
         for (const FusedMember &m : members) {
             const int N = m.N;
-            const int w = cuts(N, cuts(N, kFuseOut)), nz = cuts(N, cuts(N, depth));
+            const int w = cuts(N, cuts(N, most)), nz = cuts(N, cuts(N, depth));
             for (int z = 0; z < N; z += nz)
                 for (int y = 0; y < N; y += w)
                     for (int x = 0; x < N; x += w)
@@ -52,11 +53,17 @@ int main() {
     for (int q = 0; q < 400; ++q) {
         std::vector<FusedMember> m;
         const int n = q == 0 ? 0 : uniform(1, q % 3 == 0 ? 40 : 6);
-        const int top = q % 2 ? 160 : 70, same = q % 5 == 0 ? uniform(8, top) : 0;
+        const int top = q % 7 == 0 ? 12 : (q % 2 ? 160 : 70), same = q % 5 == 0 ? uniform(8, top) : 0;
         for (int r = 0; r < n; ++r) m.push_back(FusedMember{2 * r, same ? same : uniform(8, top)});
         const int nsm = q % 4 ? 152 : uniform(1, 152);
-        const std::vector<FusedTile> a = plan_fused(m, nsm), b = exhaustive(m, nsm);
-        bool equal = a.size() == b.size();
+        const FusedPlan plan = plan_fused(m, nsm);
+        /* blocks of 16 x 16 threads where every member fits one */
+        int largest = 0;
+        for (const FusedMember &r : m) largest = std::max(largest, r.N);
+        const bool small = n > 0 && largest <= 10;
+        const std::vector<FusedTile> &a = plan.tiles,
+                                     b = exhaustive(m, nsm * (small ? 4 : 1), small ? 10 : 26);
+        bool equal = a.size() == b.size() && plan.side == (small ? 16 : 32);
         for (size_t t = 0; equal && t < a.size(); ++t)
             equal = a[t].r == b[t].r && a[t].x0 == b[t].x0 && a[t].y0 == b[t].y0 &&
                     a[t].z0 == b[t].z0 && a[t].w == b[t].w && a[t].h == b[t].h &&

@@ -37,3 +37,21 @@ def test_last_small_member_equals_the_first(ctx, family, precision, N, members):
     assert np.isfinite(got[0]).all() and not np.array_equal(got[0], state)
     for g in got[1:]:
         assert np.array_equal(g, got[0])
+
+
+@pytest.mark.parametrize("precision", [sh.PREC_FP32, sh.PREC_FP32_KAHAN])
+def test_one_pass_blocks_of_small_members(ctx, precision):
+    """Members of up to 10^3 step in blocks of 16 x 16 threads, with a larger
+    one beside them in blocks of 32 x 32: the same bits."""
+    sizes = [8, 9, 10, 8]
+    out = []
+    for Ns in (sizes, sizes + [11]):
+        with sh.Ensemble(ctx, sh.FAMILY_AXION_LAP1, precision, Ns, [0.25] * len(Ns),
+                         [[0.5 + 0.1 * r, 0.2, 0, 0] for r in range(len(Ns))]) as E:
+            for r, n in enumerate(Ns):
+                E.write(r, axion_state(n, 0.25 * n, r))
+            E.set_time(1.0)
+            E.step(0.0625, 3)
+            out.append([E.read(r) for r in range(len(sizes))])
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
