@@ -523,17 +523,26 @@ struct FoptArgs {
     double dt;
 };
 
-/* Shared memory of the leapfrog stage kernel: the planes zc, zc + 1, zc + 2
- * with halo, and of zc - 1, zc - 2, whose halos no stencil reads any more,
- * the tile's own columns.  51 KB instead of 60 KB for five whole planes, and
- * what a block leaves goes to L1, where the loads in flight (33 words per
- * thread) have to find room: the merged stage of one 160^3 / 256^3
- * realisation takes 182 / 690 us against 231 / 809 us (0.80 of the copy rate
- * at 256^3), and 252 / 954 us with 16 KB more.  Three blocks per SM: two 189,
- * four (64 registers) 254 us. */
-template <class R>
+/* The planes zc, zc + 1, zc + 2 of the leapfrog stage kernel lie in shared
+ * memory with their halo; of zc - 1 and zc - 2, whose halos no stencil reads
+ * any more, only the tile's own columns are kept, each by its own thread: in
+ * registers where they fit beside the rest (plain FP32), else in shared memory,
+ * 51 KB in all instead of 60 KB for five whole planes.  What a block leaves
+ * goes to L1, where the loads in flight (33 words per thread) have to find
+ * room: the merged stage of one 160^3 / 256^3 realisation takes 182 / 690 us
+ * against 231 / 809 us with five planes (0.80 of the copy rate at 256^3), and
+ * 252 / 954 us with 16 KB more.  Three blocks per SM: two 189, four (64
+ * registers) 254 us.  Registers against shared memory, one step of one 160^3
+ * realisation: plain FP32 212 against 225 us, compensated 240 against 231 (the
+ * merged stage of an earlier form). */
+template <class R, bool KAHAN>
+constexpr bool below_in_registers() {
+    return sizeof(R) == 4 && !KAHAN;
+}
+template <class R, bool KAHAN>
 constexpr size_t fopt_smem() {
-    return (size_t)7 * (3 * (TY + 4) * (TX + 4) + 2 * TY * TX) * sizeof(R);
+    return (size_t)7 * (3 * (TY + 4) * (TX + 4) + (below_in_registers<R, KAHAN>() ? 0 : 2 * TY * TX)) *
+           sizeof(R);
 }
 
 /* Leapfrog kick-drift-kick stage kernel for Phi + GW tensor (7 position and
@@ -546,8 +555,9 @@ constexpr size_t fopt_smem() {
  *          rounded as the two stages round) and drifts x2 = x1 + dt vh'; v1
  *          itself is not stored.  A step of a run of steps then moves 56
  *          words per cell with compensations (28 read, 28 written) instead
- *          of 91, and evaluates the stencils once instead of twice: 340 ->
- *          231 us per step of one 160^3 realisation, FP32 + Kahan.
+ *          of 91, and evaluates the stencils once instead of twice: 184 us
+ *          per step of one 160^3 realisation, FP32 + Kahan, in place of 305
+ *          with both stages.
  * Potential: dPhi' = lap Phi + q2 Phi + q3 Phi^2 + q4 Phi^3 (p[0..2]). */
 template <class R, int STAGE, bool KAHAN>
 __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_kernel(const __grid_constant__ FoptArgs<R> a) {
@@ -555,6 +565,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
     extern __shared__ unsigned char smem_raw[];
     R(*ring)[NC][HH][W] = reinterpret_cast<R(*)[NC][HH][W]>(smem_raw);
     R(*below)[NC][TY][TX] = reinterpret_cast<R(*)[NC][TY][TX]>(ring + RING);
+    constexpr bool REG = below_in_registers<R, KAHAN>();
+    R reg1[NC] = {}, reg2[NC] = {}; /* REG: this column at planes zc - 1, zc - 2 */
 
     const FastTile tl = a.tiles[blockIdx.x];
     const RealDesc d = a.desc[tl.r];
@@ -633,6 +645,16 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
         const int s0 = (z - zb + 1) % RING; /* slot of plane zc = z - 2 */
         const int cx_ = tx + H, cy_ = ty + H;
         const int m1 = (z - zb + 1) & 1, m2 = (z - zb) & 1; /* below: planes zc - 1, zc - 2 */
+        auto low1 = [&](int c) { return REG ? reg1[c] : below[m1][c][ty][tx]; };
+        auto low2 = [&](int c) { return REG ? reg2[c] : below[m2][c][ty][tx]; };
+        auto keep = [&](int c, R v) { /* plane zc goes below */
+            if (REG) {
+                reg2[c] = reg1[c];
+                reg1[c] = v;
+            } else {
+                below[m2][c][ty][tx] = v;
+            }
+        };
         if (outp) {
             const int sp1 = (s0 + 1) % RING, sp2 = (s0 + 2) % RING;
             R acc[NC];
@@ -644,10 +666,10 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                     const double v[13] = {
                         u0, ring[s0][c][cy_][cx_ + 1], ring[s0][c][cy_][cx_ - 1],
                         ring[s0][c][cy_ + 1][cx_], ring[s0][c][cy_ - 1][cx_],
-                        ring[sp1][c][cy_][cx_], below[m1][c][ty][tx],
+                        ring[sp1][c][cy_][cx_], low1(c),
                         ring[s0][c][cy_][cx_ + 2], ring[s0][c][cy_][cx_ - 2],
                         ring[s0][c][cy_ + 2][cx_], ring[s0][c][cy_ - 2][cx_],
-                        ring[sp2][c][cy_][cx_], below[m2][c][ty][tx]};
+                        ring[sp2][c][cy_][cx_], low2(c)};
                     const int n[3] = {1, 6, 6};
                     const long long w[3] = {-90, 16, -1};
                     acc[c] = sledgehamr::utils::fixed::weighted_sum<13, 3, -2>(v, n, w, inv12dx2);
@@ -655,10 +677,10 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                 }
                 R s1 = ring[s0][c][cy_][cx_ + 1] + ring[s0][c][cy_][cx_ - 1];
                 s1 += ring[s0][c][cy_ + 1][cx_] + ring[s0][c][cy_ - 1][cx_];
-                s1 += ring[sp1][c][cy_][cx_] + below[m1][c][ty][tx];
+                s1 += ring[sp1][c][cy_][cx_] + low1(c);
                 R s2 = ring[s0][c][cy_][cx_ + 2] + ring[s0][c][cy_][cx_ - 2];
                 s2 += ring[s0][c][cy_ + 2][cx_] + ring[s0][c][cy_ - 2][cx_];
-                s2 += ring[sp2][c][cy_][cx_] + below[m2][c][ty][tx];
+                s2 += ring[sp2][c][cy_][cx_] + low2(c);
                 acc[c] = ((R)16 * s1 - s2 - (R)90 * u0) * inv12dx2;
             }
             /* 4th-order gradient of Phi */
@@ -671,8 +693,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                                       ring[s0][0][cy_][cx_ + 2], ring[s0][0][cy_][cx_ - 2]};
                 const double gy[4] = {ring[s0][0][cy_ + 1][cx_], ring[s0][0][cy_ - 1][cx_],
                                       ring[s0][0][cy_ + 2][cx_], ring[s0][0][cy_ - 2][cx_]};
-                const double gz[4] = {ring[sp1][0][cy_][cx_], below[m1][0][ty][tx],
-                                      ring[sp2][0][cy_][cx_], below[m2][0][ty][tx]};
+                const double gz[4] = {ring[sp1][0][cy_][cx_], low1(0),
+                                      ring[sp2][0][cy_][cx_], low2(0)};
                 namespace fx = sledgehamr::utils::fixed;
                 g[0] = fx::weighted_sum<4, 4, -5>(gx, n, w, inv12dx);
                 g[1] = fx::weighted_sum<4, 4, -5>(gy, n, w, inv12dx);
@@ -682,8 +704,8 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                     (ring[s0][0][cy_][cx_ + 2] - ring[s0][0][cy_][cx_ - 2])) * inv12dx;
             g[1] = ((R)8 * (ring[s0][0][cy_ + 1][cx_] - ring[s0][0][cy_ - 1][cx_]) -
                     (ring[s0][0][cy_ + 2][cx_] - ring[s0][0][cy_ - 2][cx_])) * inv12dx;
-            g[2] = ((R)8 * (ring[sp1][0][cy_][cx_] - below[m1][0][ty][tx]) -
-                    (ring[sp2][0][cy_][cx_] - below[m2][0][ty][tx])) * inv12dx;
+            g[2] = ((R)8 * (ring[sp1][0][cy_][cx_] - low1(0)) -
+                    (ring[sp2][0][cy_][cx_] - low2(0))) * inv12dx;
             }
             const R phi = ring[s0][0][cy_][cx_];
             acc[0] += phi * (q2 + phi * (q3 + phi * q4));
@@ -706,8 +728,10 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                     if (STAGE == 2) vv += hdt * acc[c];
                 }
                 a.vo[c][e] = vv;
+                const R x0 = ring[s0][c][cy_][cx_];
+                keep(c, x0);
                 if (STAGE != 1) {
-                    R xx = ring[s0][c][cy_][cx_];
+                    R xx = x0;
                     if (KAHAN) {
                         R cxx = cx_c[c];
                         kahan_add(xx, dt * vv, cxx);
@@ -718,11 +742,10 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 3 : 1) fopt_leapfrog_
                     a.xo[c][e] = xx;
                 }
             }
-        }
-        /* the plane goes below: only this thread reads its column there */
-        if (z >= zb + H)
+        } else if (active && z >= zb + H) { /* the planes below the tile's first */
 #pragma unroll
-            for (int c = 0; c < NC; ++c) below[m2][c][ty][tx] = ring[s0][c][cy_][cx_];
+            for (int c = 0; c < NC; ++c) keep(c, ring[s0][c][cy_][cx_]);
+        }
     }
 }
 
@@ -1211,7 +1234,7 @@ bool fopt_steps(sh_ensemble *E, const std::vector<void *> &cur, const std::vecto
                 int slot, double dt, int nsteps, cudaStream_t s) {
     const dim3 block(TX, TY);
     const int nt = (int)E->tiles.size();
-    const size_t shm = fopt_smem<R>();
+    const size_t shm = fopt_smem<R, KAHAN>();
     FoptArgs<R> a;
     std::memset(&a, 0, sizeof(a));
     a.desc = E->d_desc;
@@ -1424,12 +1447,12 @@ void set_smem_limits() {
     const int fsm = (int)fused_smem(kFuseSide); /* kFuseSmall needs no attribute */
     fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<true, kFuseSide>, dyn, fsm), "smem limit");
     fck(cudaFuncSetAttribute(axion_rkn4_fused_kernel<false, kFuseSide>, dyn, fsm), "smem limit");
-    const int shf = (int)fopt_smem<float>();
-    const int shd = (int)fopt_smem<double>();
+    const int shk = (int)fopt_smem<float, true>(), shf = (int)fopt_smem<float, false>();
+    const int shd = (int)fopt_smem<double, false>();
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 0, true>, at, shf), "smem limit");
-    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 1, true>, at, shf), "smem limit");
-    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 2, true>, at, shf), "smem limit");
+    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 0, true>, at, shk), "smem limit");
+    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 1, true>, at, shk), "smem limit");
+    fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 2, true>, at, shk), "smem limit");
     fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 2, false>, at, shf), "smem limit");
     fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<double, 2, false>, at, shd), "smem limit");
     fck(cudaFuncSetAttribute(fopt_leapfrog_kernel<float, 0, false>, at, shf), "smem limit");
