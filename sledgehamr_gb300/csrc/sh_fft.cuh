@@ -3,21 +3,28 @@
  * On GB300 an FP64 instruction issues at 2 lanes per clock and SM, which
  * bounds an FP64 transform; 32-bit integer adds and 32 x 32 -> 64-bit
  * multiply-adds issue at 64 and 32 lanes or so.  A line's values are
- * therefore written as integers in units of 2^-kF of a power of two above
- * the line's largest one (a block exponent per line), transformed with
+ * therefore written as integers in a unit of the line's own, transformed with
  * integer adds and products with twiddle factors of 62 fractional bits, and
  * rounded to FP64 once at the end.
  *
- * Each value and each product is rounded to the unit, an error of up to half
- * a unit wherever it is made, while the values grow with every butterfly; an
- * FP64 transform instead rounds after every operation to 2^-53 of the values
- * at that point.  With kF = 53 or 54 both end at about the same relative
- * error of the line (2-norm): 1.0e-16 to 4.7e-16 against 3.7e-16 to 7.4e-16
- * of a radix-by-radix FP64 transform on lines of 32 to 384 values.
+ * The unit is 2^-F of the power of two above the line's largest value.  Each
+ * value and each product is rounded to it, an error of up to half a unit
+ * wherever it is made, so F is as large as 64 bits allow for the line at hand
+ * (line_unit): no sum on the way exceeds the sum of the line's magnitudes, and
+ * a line with few large values gets up to 61 bits below the largest where one
+ * of even values gets 52 to 54.  An FP64 transform rounds after every operation
+ * to 2^-53 of the values at that point.  Error of a line (2-norm, 32 to 384
+ * values; noise, smooth, steep, decaying and localised lines): 0.21 to 0.47 of
+ * an FP64 transform's (pocketfft), 3.7e-17 to 9.5e-17; with frac_bits(P) for
+ * every line, up to 7 times it.  The unit costs 3 % of a 256^3 spectrum.
  *
- * Bounds, with |re|, |im| <= 2^kF and a line of P = R1 R2 <= 512 values: the
- * values grow by R1 sqrt(2) <= 2^5.1 up to the twiddle products (which need
- * |x| < 2^60) and by P sqrt(2) in all, below 2^63.
+ * Bounds, for a line z of P = R1 R2 <= 512 values whose first-stage transforms
+ * take R1 values each: the values stay below sum |z| throughout and below the
+ * largest sum |z| over R1 of them up to the twiddle products, which need 2^60.5
+ * (mul); products with constants need 2^62 and take sums of sqrt(2) times a
+ * value.  So sum |z| <= 2^61.5 and the parts' <= 2^60.5 units suffice.  With
+ * all values at the largest, frac_bits(P) holds too: P sqrt(2) 2^F < 2^63, and
+ * what enters a product then is a partial sum.
  *
  * The functions are plain C++ for host and device.
  */
@@ -140,8 +147,8 @@ inline Twiddle make_twiddle(long long j, int P) {
     split(sinl(th), w.sh, w.sl);
     return w;
 }
-/* a (c - i s) for |a| < 2^60 (then the four partial products of 2^31 units
- * stay below 2^63: 2 2^29 2^31 + sqrt(2) 2^31 2^31) */
+/* a (c - i s) for |a| <= 2^60.5 (then the four partial products of 2^31 units
+ * stay below 2^63: sqrt(2) 2^29.5 2^31 + sqrt(2) 2^31 2^31) */
 SH_HD Cx mul(Cx a, Twiddle w) {
     const int xh = (int)(a.x >> 31), xl = (int)(a.x & 0x7FFFFFFFll);
     const int yh = (int)(a.y >> 31), yl = (int)(a.y & 0x7FFFFFFFll);
@@ -247,11 +254,84 @@ SH_HD void dft(Cx (&v)[R]) {
     }
 }
 
-/* Fraction bits of a line of P values. */
+/* Fraction bits that any line of P values can have. */
 constexpr int frac_bits(int P) { return P <= 256 ? 54 : 53; }
 
-/* The value with bits (hi, lo) in units of 2^(A - 1022 - F), A the largest
- * biased exponent of the line: rounded to nearest (halves away from zero). */
+/* Of the R1 values of a line that a first-stage transform takes: the largest
+ * biased exponent e and an upper bound m of sum |re| + |im| in units of
+ * 2^(e - 1042), 2^-20 of the power of two above them. */
+struct LinePart {
+    int e;
+    unsigned m;
+};
+SH_HD unsigned shift_right(unsigned m, unsigned d) {
+#if defined(__CUDA_ARCH__)
+    unsigned r;
+    asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(m), "r"(d)); /* PTX clamps the count */
+    return r;
+#else
+    return d < 32u ? m >> d : 0u;
+#endif
+}
+/* high(n, im): high word of the real (imaginary) part of value n */
+template <int R1, class High>
+SH_HD LinePart line_part(High high) {
+    namespace fx = sledgehamr::utils::fixed;
+    int e = fx::kMinAnchor;
+#pragma unroll
+    for (int n = 0; n < 2 * R1; ++n) {
+        const int x = fx::expo(high(n >> 1, n & 1));
+        e = x > e ? x : e;
+    }
+    unsigned m = 2 * R1; /* what the shifts cut off */
+#pragma unroll
+    for (int n = 0; n < 2 * R1; ++n) {
+        const int hi = high(n >> 1, n & 1);
+        m += shift_right(((unsigned)hi & 0xFFFFFu) | 0x100000u, (unsigned)(e + 1 - fx::expo(hi)));
+    }
+    return LinePart{e, m};
+}
+
+/* The unit 2^(A - 1022 - F) of a line of P = R1 R2 values from its R2 parts:
+ * sum |z| and the parts' at most 2^61.5 and 2^60.5 of them. */
+struct LineUnit {
+    int A, F;
+};
+template <int R1, int R2, class Part>
+SH_HD LineUnit line_unit(Part part) {
+    int A = 0;
+#pragma unroll
+    for (int n = 0; n < R2; ++n) {
+        const int e = part(n).e;
+        A = e > A ? e : A;
+    }
+    unsigned sum = 0, top = 0;
+#pragma unroll
+    for (int n = 0; n < R2; ++n) {
+        const LinePart p = part(n);
+        const unsigned m = shift_right(p.m, (unsigned)(A - p.e)) + 1u;
+        sum += m;
+        top = m > top ? m : top;
+    }
+    const unsigned need = sum > 2u * top ? sum : 2u * top;
+    /* need 2^(F - 20) <= 2^61.5; sqrt(2) rounded up by 1e-6, which leaves room
+     * for the roundings */
+    const unsigned long long n = ((unsigned long long)need * 46341ull >> 15) + 1ull;
+    const int F = 81 - (63 - sledgehamr::utils::fixed::clz64(n));
+    constexpr int least = frac_bits(R1 * R2);
+    return LineUnit{A, F > 61 ? 61 : (F > least ? F : least)};
+}
+
+/* The value with bits (hi, lo) in units of 2^(A - 1022 - F), F <= 61 and A at
+ * least its biased exponent: rounded to nearest (halves away from zero). */
+SH_HD i64 to_units(double v, int A, int F) {
+    namespace fx = sledgehamr::utils::fixed;
+    const int hi = fx::hi_word(v);
+    const unsigned long long m = fx::shift_right(fx::significand<10>(hi, fx::lo_word(v)),
+                                                 (unsigned)(A + 62 - F - fx::expo(hi)));
+    const i64 r = (i64)((m + 1) >> 1); /* m: twice the units */
+    return hi < 0 ? -r : r;
+}
 template <int F>
 SH_HD i64 to_units(double v, int A) {
     namespace fx = sledgehamr::utils::fixed;
@@ -264,17 +344,20 @@ SH_HD i64 to_units(double v, int A) {
 }
 /* Back to FP64, rounded to nearest, by the conversion instruction: it takes
  * the FP64 pipe for 16 clocks of an SM, but that pipe is idle here while the
- * integer ones bound the transforms (256^3, three arrays, per axis: 504 us
- * against 568 with the conversion in integers).  to_units by conversions as
- * well makes the FP64 pipe the bound: 600 us. */
-template <int F>
-SH_HD double from_units(i64 u, int A) {
+ * integer ones bound the transforms (256^3, three arrays, per axis, all with
+ * frac_bits(P): 504 us against 568 with the conversion in integers).  to_units
+ * by conversions as well makes the FP64 pipe the bound: 600 us. */
+SH_HD double from_units(i64 u, int A, int F) {
     namespace fx = sledgehamr::utils::fixed;
     const int pw = A - 1022 - F;
     const long long b = fx::bits((double)u);
     const int e = (int)((b >> 52) & 0x7FF) + pw;
     if (u != 0 && e >= 1 && e <= 2046) return fx::from_bits(b + ((long long)pw << 52));
     return fx::to_double(u, pw);
+}
+template <int F>
+SH_HD double from_units(i64 u, int A) {
+    return from_units(u, A, F);
 }
 
 } // namespace fft

@@ -39,12 +39,14 @@ template <int R1, int R2>
 __global__ void __launch_bounds__(axis_threads<R1, R2>(), axis_threads<R1, R2>() > 256 ? 1 : 2)
     axis_kernel(double2 *__restrict__ z, long long lines, int axis,
                 const Twiddle *__restrict__ table) {
-    constexpr int P = R1 * R2, F = frac_bits(P);
+    constexpr int P = R1 * R2;
     namespace fx = sledgehamr::utils::fixed;
     extern __shared__ i64 sm[];
     constexpr int S = k1_stride<R2>();
     i64 *const sx = sm, *const sy = sm + R1 * S; /* real and imaginary parts */
-    __shared__ int top[kLines];
+    /* the parts of a line that its threads hold, and its unit */
+    __shared__ LinePart parts[R2][kLines + 1];
+    __shared__ LineUnit unit[kLines];
 
     const int tid = threadIdx.x;
     const long long l0 = (long long)blockIdx.x * kLines;
@@ -56,29 +58,26 @@ __global__ void __launch_bounds__(axis_threads<R1, R2>(), axis_threads<R1, R2>()
         return axis == 1 ? q * P * P + (l - q * P)
                          : (q / P) * P * P * P + (q % P) * P + (l - q * P);
     };
-    if (tid < kLines) top[tid] = fx::kMinAnchor;
-
     int line = axis == 0 ? tid / R2 : tid % kLines;
     const int n2 = axis == 0 ? tid % R2 : tid / kLines;
     bool in = line < kLines && n2 < R2 && l0 + line < lines;
     Cx v[R1];
     double2 a[R1];
-    int e = 0;
     if (in) {
         const double2 *const p = z + first(l0 + line) + n2 * stride;
 #pragma unroll
         for (int n = 0; n < R1; ++n) a[n] = p[(long long)(n * R2) * stride];
-#pragma unroll
-        for (int n = 0; n < R1; ++n)
-            e = max(e, max(fx::expo(fx::hi_word(a[n].x)), fx::expo(fx::hi_word(a[n].y))));
+        parts[n2][line] =
+            line_part<R1>([&](int n, int im) { return fx::hi_word(im ? a[n].y : a[n].x); });
     }
     __syncthreads();
-    if (in) atomicMax(&top[line], e);
-    __syncthreads();
     if (in) {
-        const int A = top[line];
+        const LineUnit u =
+            line_unit<R1, R2>([&](int n) { return parts[n][line]; });
+        if (n2 == 0) unit[line] = u;
 #pragma unroll
-        for (int n = 0; n < R1; ++n) v[n] = Cx{to_units<F>(a[n].x, A), to_units<F>(a[n].y, A)};
+        for (int n = 0; n < R1; ++n)
+            v[n] = Cx{to_units(a[n].x, u.A, u.F), to_units(a[n].y, u.A, u.F)};
         dft<R1>(v);
 #pragma unroll
         for (int k = 0; k < R1; ++k) {
@@ -97,14 +96,14 @@ __global__ void __launch_bounds__(axis_threads<R1, R2>(), axis_threads<R1, R2>()
     for (int n = 0; n < R2; ++n)
         w[n] = Cx{sx[k1 * S + n * (kLines + 1) + line], sy[k1 * S + n * (kLines + 1) + line]};
     dft<R2>(w);
-    const int A = top[line];
+    const int A = unit[line].A, F = unit[line].F;
     double2 *const p = z + first(l0 + line) + k1 * stride;
     const bool finite = A != 0x7FF; /* a line holding NaN or infinity gives NaN */
 #pragma unroll
     for (int k = 0; k < R2; ++k) {
         const double nan = fx::from_bits(0x7FF8000000000000ll);
         p[(long long)(k * R1) * stride] =
-            finite ? make_double2(from_units<F>(w[k].x, A), from_units<F>(w[k].y, A))
+            finite ? make_double2(from_units(w[k].x, A, F), from_units(w[k].y, A, F))
                    : make_double2(nan, nan);
     }
 }
@@ -116,7 +115,7 @@ template <int R1, int R2>
 cudaError_t launch_axis(double2 *z, long long lines, int axis, const Twiddle *table,
                         cudaStream_t s) {
     constexpr size_t smem = axis_smem<R1, R2>();
-    if constexpr (smem + kLines * sizeof(int) > 48 * 1024) {
+    if constexpr (smem + (kLines + 1) * (R2 * sizeof(LinePart) + sizeof(LineUnit)) > 48 * 1024) {
         const cudaError_t e =
             cudaFuncSetAttribute(axis_kernel<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
