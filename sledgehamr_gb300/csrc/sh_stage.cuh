@@ -159,6 +159,11 @@ __global__ void __launch_bounds__(kTileX *kTileY, (stage_min_blocks<GW, KO, H::k
                     r[n] += sledgehamr::kernels::KreissOligerDissipation<KO>(
                         st, i, j, k, n, a.dx, a.ko_strength[n]);
             });
+            if constexpr (H::kNScalars % 2 == 1) { /* a field without a partner */
+                constexpr int n = H::kNScalars - 1;
+                r[n] += sledgehamr::kernels::KreissOligerDissipation<KO>(st, i, j, k, n, a.dx,
+                                                                        a.ko_strength[n]);
+            }
         }
 
         const long long lc = (i - glo.x) + (j - glo.y) * gx + (k - glo.z) * gxy;

@@ -65,3 +65,17 @@ def test_shipped_rhs_inside_a_users_project(tmp_path):
             driven = ctx.evolve_periodic("DrivenStrings", integ, st, params=[0.8, 0.3, 5.0], **kw)
             assert rel_l2(driven, want) > 1e-3
     """)
+
+
+def test_dissipation_of_an_odd_number_of_fields(tmp_path):
+    """Three fields with one state and one strength stay equal, bit for bit,
+    and are smoothed, for both orders."""
+    run_with(library_with("odd_project.cu", tmp_path), """
+        N = 16
+        st = np.repeat(axion_state(N, N * 0.25)[:1], 3, axis=0)
+        for order in (2, 3):
+            got = ctx.evolve_periodic("ThreeFields", sh.LSSSPRK3, st, t0=1.0, dt=0.05, dx=0.25,
+                                      nsteps=3, nghost=3, ko_order=order, ko_strength=[0.3] * 3)
+            assert not np.array_equal(got[0], st[0])
+            assert np.array_equal(got[1], got[0]) and np.array_equal(got[2], got[0]), order
+    """)
