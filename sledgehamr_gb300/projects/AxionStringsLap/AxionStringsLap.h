@@ -33,18 +33,18 @@
         const double psi2 = state(i, j, k, Scalar::Psi2);                      \
         const double pi1 = state(i, j, k, Scalar::Pi1);                        \
         const double pi2 = state(i, j, k, Scalar::Pi2);                        \
-        const double mod2 = psi1 * psi1 + psi2 * psi2;                         \
+        const double v = sh_axion::potential(s, psi1, psi2);                   \
         rhs(i, j, k, Scalar::Psi1) = pi1;                                      \
         rhs(i, j, k, Scalar::Psi2) = pi2;                                      \
         rhs(i, j, k, Scalar::Pi1) = sh_axion::accel(                           \
             s, psi1, pi1,                                                      \
-            sledgehamr::utils::Laplacian<ORDER>(state, i, j, k, Scalar::Psi1, dx * dx), mod2); \
+            sledgehamr::utils::Laplacian<ORDER>(state, i, j, k, Scalar::Psi1, dx * dx), v); \
         rhs(i, j, k, Scalar::Pi2) = sh_axion::accel(                           \
             s, psi2, pi2,                                                      \
-            sledgehamr::utils::Laplacian<ORDER>(state, i, j, k, Scalar::Psi2, dx * dx), mod2); \
+            sledgehamr::utils::Laplacian<ORDER>(state, i, j, k, Scalar::Psi2, dx * dx), v); \
     }                                                                          \
     inline void StageParams(double *params, const double time) {               \
-        sh_axion::store_constants(params, time, params[0], params[1]);         \
+        sh_axion::store_constants(params, time);                               \
     }                                                                          \
     SH_AXION_STRING_TAGGING                                                    \
     SLEDGEHAMR_FINISH_SETUP                                                    \

@@ -22,17 +22,17 @@ Rhs(const amrex::Array4<double> &rhs, const amrex::Array4<const double> &state, 
     const sh_axion::StageConstants s = sh_axion::constants(params, time, params[0], 0.56233);
     const double psi1 = state(i, j, k, Scalar::Psi1), psi2 = state(i, j, k, Scalar::Psi2);
     const double pi1 = state(i, j, k, Scalar::Pi1), pi2 = state(i, j, k, Scalar::Pi2);
-    const double mod2 = psi1 * psi1 + psi2 * psi2;
+    const double v = sh_axion::potential(s, psi1, psi2);
     const double lap1 = sledgehamr::utils::Laplacian<2>(state, i, j, k, Scalar::Psi1, dx * dx);
     const double lap2 = sledgehamr::utils::Laplacian<2>(state, i, j, k, Scalar::Psi2, dx * dx);
     rhs(i, j, k, Scalar::Psi1) = pi1;
     rhs(i, j, k, Scalar::Psi2) = pi2;
-    rhs(i, j, k, Scalar::Pi1) = sh_axion::accel(s, psi1, pi1, lap1, mod2);
-    rhs(i, j, k, Scalar::Pi2) = sh_axion::accel(s, psi2, pi2, lap2, mod2);
+    rhs(i, j, k, Scalar::Pi1) = sh_axion::accel(s, psi1, pi1, lap1, v);
+    rhs(i, j, k, Scalar::Pi2) = sh_axion::accel(s, psi2, pi2, lap2, v);
 }
 
 inline void StageParams(double *params, const double time) {
-    sh_axion::store_constants(params, time, params[0], 0.56233);
+    sh_axion::store_constants(params, time);
 }
 
 SLEDGEHAMR_FINISH_SETUP
