@@ -72,8 +72,8 @@ WORDS_PER_CELL_UPDATE = 40
 # launch of the benchmark by the cells it updates.  AMR: level 1 of the AMR
 # run at N0 = 128 (5.60 GB for 11,812,352 cells); 128^3 level: the three
 # launches of one step of `--case single`, ghost images written by the stage
-# kernel (597.5 MB for 2,097,152 cells).
-TRAFFIC_B_PER_CELL_UPDATE = {"amr": 474.0, "single": 284.9}
+# kernel (602.6 MB for 2,097,152 cells).
+TRAFFIC_B_PER_CELL_UPDATE = {"amr": 474.0, "single": 287.3}
 # whole-job end-to-end runs of the 128^3 level (the median is reported)
 E2E_JOBS = 3
 
@@ -865,8 +865,8 @@ def timed_steps(step, steps, warmup, stream, flush, clk=None, before=None):
 # kernels (ncu executed-instruction counters of the three launches of one RKN4
 # step divided by the cells): the 7-point kernel of the 128^3 level
 # (`--case single`) and the 13-point kernel on levels of eight-plane tiles
-# (256^3 in 64^3 boxes), which form their scale once per column.
-FP64_INSTR_PER_CELL_UPDATE = {"single": 41.25, "amr": 47.625}
+# (256^3 in 32^3 boxes), which form their scale once per column.
+FP64_INSTR_PER_CELL_UPDATE = {"single": 44.25, "amr": 50.625}
 
 
 def fp64_probe(device):

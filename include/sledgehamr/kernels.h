@@ -60,11 +60,13 @@ KreissOligerDissipation(const amrex::Array4<double const> &state, const int i,
                         const double dissipation_strength) {
     static_assert(Order == 2 || Order == 3, "KO dissipation order 2 or 3");
 #if defined(__CUDA_ARCH__) && !defined(SH_STENCIL_FP64)
-    /* the three axes' differences as one weighted sum of the rings, exact in
-     * integers (2^53 times 48 or 192: headroom of 4 and 2 bits), and a
+    /* the three axes' differences as one weighted sum of the rings in integers
+     * (2^53 times 48 or 192: headroom of 4 and 2 bits), rounded once, and a
      * product with a factor formed once per thread: the FP64 form below
-     * takes 17 adds and two divisions per component on the narrow FP64
-     * pipe */
+     * takes 17 adds and two divisions per component on the narrow FP64 pipe.
+     * Values are cut off 4 and 2 bits below the last place of the stencil's
+     * largest one, and below 2^-895; a stencil holding infinity gives NaN
+     * (sh_fixed_stencil.h) */
     if constexpr (Order == 2)
         return utils::detail::rings_fixed<2, -4>(
             state, i, j, k, c,

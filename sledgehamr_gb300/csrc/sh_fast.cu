@@ -346,10 +346,10 @@ __global__ void __launch_bounds__(TX *TY, sizeof(R) == 4 ? 5 : 1) axion_rkn4_ker
  *
  * 32 x 32 threads, so up to 26 x 26 cells a block and one block per SM (16 x
  * 16 for members of up to 10^3 cells, sh_fuse_plan.h); 32 x 24 threads measured
- * 11 %, two blocks of 32 x 16 8 % slower at 256^3.  Bound by instruction issue (77 % of the slots; sm_100's
- * packed FP32 instructions measured the same).  Per step, FP32 + Kahan: one
- * 256^3 realisation 560 -> 285 us, a mix of eight from 32^3 to 128^3 262 ->
- * 127 us. */
+ * 11 %, two blocks of 32 x 16 8 % slower at 256^3.  Bound by instruction issue
+ * (77 % of the slots at 256^3; packed FP32 instructions measured the same).  Per
+ * step, FP32 + Kahan: one 256^3 realisation 560 -> 285 us, a mix of eight from
+ * 32^3 to 128^3 262 -> 127 us. */
 constexpr size_t fused_smem(int side) {
     /* stage positions [2][3] and momenta [4] of a plane of threads, pairs */
     return (size_t)(2 * 3 + 4) * side * side * sizeof(float2);

@@ -9,7 +9,8 @@
 namespace sh {
 namespace fft {
 
-/* Whether transform3 takes P^3 arrays: P a product of two radices it has. */
+/* Whether transform3 takes P^3 arrays: P one of the 19 sizes instantiated in
+ * sh_fft_small.cu, sh_fft_medium.cu and sh_fft_large.cu, up to 384. */
 bool supported(int P);
 /* Twiddle factors exp(-2 pi i j / P), j < P, on the device (cudaFree'd by the
  * caller); nullptr when the allocation fails. */

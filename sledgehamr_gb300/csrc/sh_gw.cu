@@ -507,9 +507,9 @@ cudaError_t gw_spectrum_packed(GwCache &cache, cudaStream_t stream, int P, int N
                                const std::function<void(int, double2 *)> &pack) {
     cache.prepare(P, unbinned, projection_type);
     const long long nfull = (long long)P * P * P;
-    /* the library's own transforms where P is a product of two of their
-     * radices, cuFFT's otherwise (256^3, three arrays: 10.3 ms with cuFFT,
-     * which is bound by the FP64 pipe, 1.5 ms in integers) */
+    /* the library's own transforms at the sizes that they have, cuFFT's
+     * otherwise (256^3, three arrays: 10.3 ms with cuFFT, which is bound by
+     * the FP64 pipe, 1.6 ms in integers) */
     cufftHandle plan = 0;
     const fft::Twiddle *table = nullptr;
     if (fft::supported(P)) {

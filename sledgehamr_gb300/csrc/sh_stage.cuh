@@ -67,8 +67,8 @@ constexpr int stage_min_blocks() {
 
 /* EPI: the epilogue, or kEpiAny where it is taken from the arguments at run
  * time.  The instantiations for the RKN4 and leapfrog stages leave out the
- * switch and the loops over the earlier K: 663 -> 555 warp instructions per
- * 32 cells of an intermediate RKN4 stage (with the leaner integer sums). */
+ * switch and the loops over the earlier K; an intermediate RKN4 stage of the
+ * 7-point kernel issues 597 warp instructions per 32 cells. */
 template <class H, bool GW, int KO, bool SP = false, int EPI = kEpiAny>
 __global__ void __launch_bounds__(kTileX *kTileY, (stage_min_blocks<GW, KO, H::kReach>()))
     stage_kernel(const __grid_constant__ StageArgs a) {

@@ -81,7 +81,8 @@ __device__ __forceinline__ void st_cells(float *p, int o, const float (&x)[V]) {
  * 8-byte words, 7 loads per component and pair instead of 18 with 13 points,
  * and 200 instructions per cell row become 90; it needs rows of an even number
  * of cells behind an even number of ghost cells in all boxes (L->x_pairs, so
- * that every pair lies on an 8-byte boundary), and V = 1 takes the others.
+ * that every pair lies on an 8-byte boundary), and V = 1 takes the others, the
+ * 7-point levels of one ghost cell among them.
  * 64 boxes of 64^3, 13 points, stages 0, 1, 2: V = 1 with the next plane's
  * words prefetched 158, 178, 340 us; V = 2 in 32-cell rows and 8 planes 143,
  * 159, 302 us, in 64-cell rows and 4 planes 133, 147, 275 us (floors at

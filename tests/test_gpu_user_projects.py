@@ -1,5 +1,5 @@
-"""Projects of a user's own, compiled and linked with the library's objects
-as INTEGRATION describes, stepped on the GPU in a process of their own."""
+"""Projects of a user's own, compiled and linked with the library's objects,
+stepped on the GPU in a process of their own."""
 import glob
 import os
 import shutil
