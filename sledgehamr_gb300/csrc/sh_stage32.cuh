@@ -75,7 +75,7 @@ __device__ __forceinline__ void st_cells(float *p, int o, const float (&x)[V]) {
  * restrict-qualified pointers (every buffer of a stage is distinct).  The sums
  * are formed in the order of the ensemble kernels (x+, x-, y+, y-, z+, z-).
  *
- * Memory bounds the stages (8, 10 and 22 words per cell; DRAM moves 14-17%
+ * Memory bounds the stages (8, 10 and 22 words per cell; DRAM moves 11-12%
  * more, for the ghost cells), through the loads that wait and the sectors that
  * a 128-byte row 8 bytes off its boundary touches twice.  V = 2 reads pairs as
  * 8-byte words, 7 loads per component and pair instead of 18 with 13 points,
