@@ -14,7 +14,7 @@ bool supported(int P) {
     return false;
 }
 
-Twiddle *make_table(int P) {
+Twiddle *make_table(int P, cudaStream_t s) {
     std::vector<Twiddle> h(P);
     for (int j = 0; j < P; ++j) h[j] = make_twiddle(j, P);
     Twiddle *d = nullptr;
@@ -22,7 +22,10 @@ Twiddle *make_table(int P) {
         cudaGetLastError();
         return nullptr;
     }
-    if (cudaMemcpy(d, h.data(), P * sizeof(Twiddle), cudaMemcpyHostToDevice) != cudaSuccess) {
+    /* in stream order: a copy on the default stream is not ordered with a
+     * non-blocking one, and may end after its call returns */
+    if (cudaMemcpyAsync(d, h.data(), P * sizeof(Twiddle), cudaMemcpyHostToDevice, s) !=
+        cudaSuccess) {
         cudaGetLastError();
         cudaFree(d);
         return nullptr;

@@ -13,8 +13,8 @@ namespace fft {
  * sh_fft_small.cu, sh_fft_medium.cu and sh_fft_large.cu, up to 384. */
 bool supported(int P);
 /* Twiddle factors exp(-2 pi i j / P), j < P, on the device (cudaFree'd by the
- * caller); nullptr when the allocation fails. */
-Twiddle *make_table(int P);
+ * caller), written in stream order; nullptr when the allocation fails. */
+Twiddle *make_table(int P, cudaStream_t s);
 /* In-place forward transforms of n complex FP64 P^3 arrays, one after the
  * other in z (element (x, y, z) of array q at ((q P + z) P + y) P + x),
  * unnormalised; table from make_table(P).  Three launches. */

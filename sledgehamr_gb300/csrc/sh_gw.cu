@@ -377,10 +377,15 @@ __global__ void scalar_power_kernel(const double2 *F, int P, double *out) {
     }
 }
 
+template <class T>
+bool upload(T *d, const std::vector<T> &h, cudaStream_t s) {
+    return cudaMemcpyAsync(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s) ==
+           cudaSuccess;
+}
 } // namespace
 
 /* Builds (or reuses) the bin lists of a P^3 spectrum. */
-void GwCache::prepare(int P, int unbinned, int projection_type) {
+void GwCache::prepare(int P, int unbinned, int projection_type, cudaStream_t s) {
     ++clock;
     for (GwBins &b : bins)
         if (b.P == P && b.unbinned == unbinned && b.projection_type == projection_type) {
@@ -410,7 +415,9 @@ void GwCache::prepare(int P, int unbinned, int projection_type) {
     if (cudaMalloc(&g.d_off, lists.off.size() * sizeof(long long)) != cudaSuccess ||
         cudaMalloc(&g.d_cells, lists.cells.size() * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&g.d_itk, itk.size() * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&g.d_itk32, itk32.size() * sizeof(float)) != cudaSuccess) {
+        cudaMalloc(&g.d_itk32, itk32.size() * sizeof(float)) != cudaSuccess ||
+        !upload(g.d_off, lists.off, s) || !upload(g.d_cells, lists.cells, s) ||
+        !upload(g.d_itk, itk, s) || !upload(g.d_itk32, itk32, s)) {
         cudaGetLastError();
         cudaFree(g.d_off);
         cudaFree(g.d_cells);
@@ -418,10 +425,6 @@ void GwCache::prepare(int P, int unbinned, int projection_type) {
         cudaFree(g.d_itk32);
         throw std::bad_alloc();
     }
-    cudaMemcpy(g.d_off, lists.off.data(), lists.off.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    cudaMemcpy(g.d_cells, lists.cells.data(), lists.cells.size() * sizeof(int), cudaMemcpyHostToDevice);
-    cudaMemcpy(g.d_itk, itk.data(), itk.size() * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(g.d_itk32, itk32.data(), itk32.size() * sizeof(float), cudaMemcpyHostToDevice);
     bins.push_back(std::move(g));
     cur = &bins.back();
 }
@@ -463,7 +466,7 @@ bool GwCache::plan(int P, int kind, cufftHandle *out) {
     return true;
 }
 
-const fft::Twiddle *GwCache::table(int P) {
+const fft::Twiddle *GwCache::table(int P, cudaStream_t s) {
     ++clock;
     for (Table &t : tables)
         if (t.P == P) {
@@ -480,7 +483,7 @@ const fft::Twiddle *GwCache::table(int P) {
     Table t;
     t.P = P;
     t.used = clock;
-    t.d = fft::make_table(P);
+    t.d = fft::make_table(P, s);
     if (t.d) tables.push_back(t);
     return t.d;
 }
@@ -505,7 +508,7 @@ cudaError_t gw_spectrum_packed(GwCache &cache, cudaStream_t stream, int P, int N
                                double *bins_dev, int *nbins, long long *launches,
                                std::string &err,
                                const std::function<void(int, double2 *)> &pack) {
-    cache.prepare(P, unbinned, projection_type);
+    cache.prepare(P, unbinned, projection_type, stream);
     const long long nfull = (long long)P * P * P;
     /* the library's own transforms at the sizes that they have, cuFFT's
      * otherwise (256^3, three arrays: 10.3 ms with cuFFT, which is bound by
@@ -513,7 +516,7 @@ cudaError_t gw_spectrum_packed(GwCache &cache, cudaStream_t stream, int P, int N
     cufftHandle plan = 0;
     const fft::Twiddle *table = nullptr;
     if (fft::supported(P)) {
-        table = cache.table(P);
+        table = cache.table(P, stream);
         if (!table) throw std::bad_alloc();
     } else {
         if (!cache.plan(P, GwCache::kPlanZ2Z3, &plan)) {
@@ -556,7 +559,7 @@ cudaError_t gw_spectrum_packed32(GwCache &cache, cudaStream_t stream, int P, int
                                  double *bins_dev, int *nbins, long long *launches,
                                  std::string &err,
                                  const std::function<void(int, float2 *)> &pack) {
-    cache.prepare(P, unbinned, projection_type);
+    cache.prepare(P, unbinned, projection_type, stream);
     const int H = P / 2 + 1;
     const long long nfull = (long long)P * P * P;
     const long long nhalf = (long long)H * P * P;
@@ -595,7 +598,7 @@ cudaError_t scalar_spectrum_packed(GwCache &cache, cudaStream_t stream, int P, d
                                    long long *launches, std::string &err,
                                    const std::function<void(double *)> &pack) {
     /* unbinned bins of k^2 (the k-map of the entry is not used) */
-    cache.prepare(P, 1, 2);
+    cache.prepare(P, 1, 2, stream);
     const int H = P / 2 + 1;
     const long long nreal = (long long)P * P * P;
     const long long ncplx = (long long)H * P * P;

@@ -54,12 +54,13 @@ struct GwCache {
     GwBins *cur = nullptr;
     /* k^2 of the bins of the last prepared kind */
     const std::vector<long long> &ks() const { return cur->ks; }
-    void prepare(int P, int unbinned, int projection_type);
+    /* tables are written in the order of the stream that reads them */
+    void prepare(int P, int unbinned, int projection_type, cudaStream_t s);
     /* cuFFT plan of a kind for P^3 (created on first use); false if cuFFT
      * fails */
     bool plan(int P, int kind, cufftHandle *out);
     /* twiddle table of P (made on first use; nullptr without memory) */
-    const fft::Twiddle *table(int P);
+    const fft::Twiddle *table(int P, cudaStream_t s);
     void release();
 };
 

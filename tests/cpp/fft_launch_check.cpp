@@ -2,11 +2,13 @@
  * for the CUDA runtime that keeps, as the runtime does, the dynamic
  * shared-memory limit of a kernel per device.  For every grid size: the first
  * transform of a process on device 0, then one on device 1, then one whose
- * limit cannot be set and the same again.  Linked with the library's objects;
- * no GPU. */
+ * limit cannot be set and the same again; and the stream on which the twiddle
+ * factors are copied.  Linked with the library's objects; no GPU. */
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
+#include <cstring>
 #include <map>
 #include <utility>
 
@@ -18,6 +20,7 @@ bool refuse = false; /* setting a limit fails */
 std::map<std::pair<int, const void *>, int> limit;
 cudaError_t last = cudaSuccess;
 long long launched = 0;
+cudaStream_t copied_on = nullptr;
 struct {
     dim3 grid, block;
     size_t smem;
@@ -68,9 +71,24 @@ cudaError_t cudaGetLastError() {
     last = cudaSuccess;
     return e;
 }
-cudaError_t cudaMalloc(void **, size_t) { return cudaErrorMemoryAllocation; }
-cudaError_t cudaFree(void *) { return cudaSuccess; }
-cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind) { return cudaSuccess; }
+cudaError_t cudaMalloc(void **p, size_t n) {
+    *p = std::malloc(n);
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+    std::free(p);
+    return cudaSuccess;
+}
+/* a copy on the default stream: other streams' kernels do not wait for it */
+cudaError_t cudaMemcpy(void *, const void *, size_t, cudaMemcpyKind) {
+    copied_on = nullptr;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *h, size_t n, cudaMemcpyKind, cudaStream_t s) {
+    std::memcpy(d, h, n);
+    copied_on = s;
+    return cudaSuccess;
+}
 }
 
 int main() {
@@ -102,6 +120,15 @@ int main() {
             check(P, "the call after it", true);
         }
     }
+    /* the twiddle factors, in the order of the stream that reads them */
+    const cudaStream_t stream = (cudaStream_t)&sizes;
+    sh::fft::Twiddle *const t = sh::fft::make_table(64, stream);
+    const sh::fft::Twiddle want = sh::fft::make_twiddle(5, 64);
+    if (!t || copied_on != stream || std::memcmp(&t[5], &want, sizeof want) != 0) {
+        std::printf("twiddle factors not written on the stream\n");
+        ++bad;
+    }
+    cudaFree(t);
     std::printf("%d sizes\n", sizes);
     return bad || sizes == 0;
 }
