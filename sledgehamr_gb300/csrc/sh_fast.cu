@@ -1512,7 +1512,7 @@ double read_time(sh_ensemble *E) {
 
 void alloc_error_flag(sh_ensemble *E) {
     fck(cudaMalloc(&E->d_err, sizeof(int)), "error flag");
-    fck(cudaMemset(E->d_err, 0, sizeof(int)), "error flag clear");
+    fck(cudaMemsetAsync(E->d_err, 0, sizeof(int), est(E)), "error flag clear");
 }
 
 } // namespace
@@ -1560,7 +1560,7 @@ int sh_ensemble_create(sh_ctx *ctx, int family, int precision, int nreal, const 
                 void *p = nullptr;
                 fck(cudaMalloc(&p, bytes), "ensemble allocation");
                 v.push_back(p);
-                fck(cudaMemset(p, 0, bytes), "ensemble clear");
+                fck(cudaMemsetAsync(p, 0, bytes, est(E)), "ensemble clear");
             }
         };
         alloc(E->A, E->ncomp);
@@ -1569,7 +1569,7 @@ int sh_ensemble_create(sh_ctx *ctx, int family, int precision, int nreal, const 
         alloc(E->K, family == SH_FAMILY_FOPT_GW ? 7 : 4);
         E->A0 = E->A[0];
         fck(cudaMalloc(&E->d_time, 2 * sizeof(double)), "time");
-        fck(cudaMemset(E->d_time, 0, 2 * sizeof(double)), "time clear");
+        fck(cudaMemsetAsync(E->d_time, 0, 2 * sizeof(double), est(E)), "time clear");
         fck(cudaMalloc(&E->d_counts, nreal * sizeof(unsigned long long)), "counts");
         E->counts_cap = nreal;
         alloc_error_flag(E);
@@ -2045,7 +2045,7 @@ int sh_ensemble_create_pool(sh_ctx *ctx, int family, int precision, long long ca
         E->A0 = E->A[0];
         E->free_ext[0] = capacity_cells;
         fck(cudaMalloc(&E->d_time, 2 * sizeof(double)), "time");
-        fck(cudaMemset(E->d_time, 0, 2 * sizeof(double)), "time clear");
+        fck(cudaMemsetAsync(E->d_time, 0, 2 * sizeof(double), est(E)), "time clear");
         alloc_error_flag(E);
     });
     if (rc != SH_OK) {
