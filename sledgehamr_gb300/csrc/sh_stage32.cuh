@@ -125,9 +125,11 @@ __global__ void __launch_bounds__(kThreads / V, V == 1 ? (STAGE == 2 ? 10 : 16)
 #pragma unroll
         for (int d = 0; d < 2 * R; ++d) ld_cells<V>(w[c][d], st + c * gvol, o + (d - R) * gxy);
     for (int n = kend - t.z0; n >= 0; --n, o += gxy) {
-        /* the next cell's y0 asked into L1 while this one is computed (27
-         * boxes of 63^3: 77.8 us against 82.5 in this form, and slower or the
-         * same in the others) */
+        /* the next cell's y0 asked into L1 while this one is computed, in the
+         * form that gains by it on large levels: a step of one 192^3 level of
+         * three ghost cells 319 us against 325, of 27 boxes of 63^3 405
+         * against 407, of 96^3 63.4 against 62.5; in every form of V = 1 the
+         * 7-point steps of 160^3 and more take 4 % longer */
         if constexpr (V == 1 && ORDER == 2 && STAGE == 1) {
             if (n > 0) {
 #pragma unroll
